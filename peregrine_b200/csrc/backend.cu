@@ -2,6 +2,7 @@
 // calls of the reference ABI and the device-resident MoE layer.  Declarations
 // and the reference lines each entry point replaces are in
 // include/peregrine_b200.h.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -13,8 +14,8 @@
 #include "kernels.cuh"
 #include "kernels_mma.cuh"
 #include "kernels_tile.cuh"
-#include "kernels_umma.cuh"
 #include "kernels_block.cuh"
+#include "kernels_fold.cuh"
 #include "kernels_decode.cuh"
 #include "kernels_ep.cuh"
 #include "w4_host.h"
@@ -607,25 +608,7 @@ static int tile_launch_t(Ctx *c, const GemvParams &P) {
     return launch(kfn, dim3(n_oblk, P.tile_rb), dim3(kTileThreads), (size_t)kTileSmemBytes, c->stream,
                   "w4a8 tile kernel launch", P);
 }
-template <bool GROUPED, int BPG>
-static int umma_launch_t(Ctx *c, const GemvParams &P) {
-    auto kfn = ffn_w4a8_umma_kernel<GROUPED, BPG>;
-    if (!ensure_smem(c, kfn, (size_t)kUmSmemBytes, "tcgen05 kernel shared-memory opt-in")) return 0;
-    const int n_oblk = (P.mode == 0) ? (P.ntile + 3) / 4 : (P.ntile + 7) / 8;
-    return launch(kfn, dim3(n_oblk, P.tile_rb), dim3(kUmThreads), (size_t)kUmSmemBytes, c->stream,
-                  "w4a8 tcgen05 kernel launch", P);
-}
 static int tile_launch(Ctx *c, const GemvParams &P, bool grouped, int bpg) {
-    if (P.umma) {
-        if (!grouped) return umma_launch_t<false, 1>(c, P);
-        switch (bpg) {
-            case 1: return umma_launch_t<true, 1>(c, P);
-            case 2: return umma_launch_t<true, 2>(c, P);
-            case 4: return umma_launch_t<true, 4>(c, P);
-            case 8: return umma_launch_t<true, 8>(c, P);
-        }
-        return fail("w4a8 tcgen05 kernel: unsupported group size");
-    }
     if (!grouped) return tile_launch_t<false, 1>(c, P);
     switch (bpg) {
         case 1: return tile_launch_t<true, 1>(c, P);
@@ -634,6 +617,73 @@ static int tile_launch(Ctx *c, const GemvParams &P, bool grouped, int bpg) {
         case 8: return tile_launch_t<true, 8>(c, P);
     }
     return fail("w4a8 tile kernel: unsupported group size");
+}
+
+// ---- fold kernel (tcgen05)
+// Can it hold the launch at all: its slot table, and for per-row scales the whole row's integer dot, which
+// has to stay exact in the fp32 accumulator (8 * 128 * K <= 2^24).
+static bool fold_fits(const W4Layout &L, int slots_max) {
+    return slots_max <= kFoMaxSlots && (L.grouped || L.kp <= 16384);
+}
+// Is it the faster one for `slots` experts with `rows` rows together and at most `max_rows` each?  Its items are
+// long pipelines (256 weight rows, all of K): it needs K of 8 chunks (measured at 301 tokens: 6 chunks 173 us
+// against 160 for the tile kernel, 8 chunks 160 against 170 at 128 tokens) and items for most of the CTAs
+// (one 2048 x 8192 matrix at 100 rows: 64 items, 44 us against 40 for the small-batch kernel; 6144 x 12288:
+// 96 items, 69 against 94), and below 32 rows most of its columns are padding (6144 x 32000, 12 rows: 86 us
+// against 72; 32 rows: 86 against 93; 64 rows: 100 against 147).
+static bool fold_pays(Ctx *c, const W4Layout &L, int mode, int max_rows, long long rows, int slots) {
+    const long long n_ob = mode == 0 ? (L.ntile + 7) / 8 : (L.ntile + 15) / 16;
+    const long long units = std::max<long long>(slots, (rows + kFoTok - 1) / kFoTok);
+    return fold_fits(L, slots) && L.nchunk >= 8 && max_rows >= 32 && rows >= 16LL * slots && 5 * n_ob * units >= 3LL * c->sms;
+}
+static size_t act_f16_bytes(const W4Layout &L, size_t rows) { return rows * (size_t)L.kp * 2; }
+
+// fp16 activation rows [rows][kp] as boxes of 64 elements x 32 rows, 128-byte swizzle.
+static int fold_map_make(CUtensorMap *m, const void *base, long long rows, int kp) {
+    typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const EncodeFn enc = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult st;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &st) != cudaSuccess ||
+            st != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return (EncodeFn)fn;
+    }();
+    if (!enc) return fail("fold kernel: the driver has no tensor map encoder");
+    const cuuint64_t dims[2] = {(cuuint64_t)kp, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)kp * 2};
+    const cuuint32_t box[2] = {kFoXGroup, kFoXBoxRows}, es[2] = {1, 1};
+    if (enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return fail("fold kernel: tensor map refused");
+    return 1;
+}
+template <int TOK, bool GROUPED, int BPG>
+static int fold_launch_t(Ctx *c, const GemvParams &P, const CUtensorMap &map) {
+    auto kfn = ffn_w4a8_fold_kernel<TOK, GROUPED, BPG>;
+    if (!ensure_smem(c, kfn, (size_t)fo_smem_bytes(TOK), "fold kernel shared-memory opt-in")) return 0;
+    return launch(kfn, dim3(c->sms), dim3(kFoThreads), (size_t)fo_smem_bytes(TOK), c->stream, "w4a8 fold kernel launch",
+                  map, P);
+}
+template <int TOK>
+static int fold_launch_g(Ctx *c, const GemvParams &P, const CUtensorMap &map, bool grouped, int bpg) {
+    if (!grouped) return fold_launch_t<TOK, false, 1>(c, P, map);
+    switch (bpg) {
+        case 1: return fold_launch_t<TOK, true, 1>(c, P, map);
+        case 2: return fold_launch_t<TOK, true, 2>(c, P, map);
+        case 4: return fold_launch_t<TOK, true, 4>(c, P, map);
+        case 8: return fold_launch_t<TOK, true, 8>(c, P, map);
+    }
+    return fail("w4a8 fold kernel: unsupported group size");
+}
+static int fold_launch(Ctx *c, const GemvParams &P, const W4Layout &L) {
+    CUtensorMap map;
+    if (!fold_map_make(&map, P.xh, P.xh_rows, L.kp)) return 0;
+    return fold_launch_g<kFoTok>(c, P, map, L.grouped != 0, L.bpg);
 }
 
 // Fills the layout-dependent fields and launches.  `max_rows` bounds the rows of any slot:
@@ -663,6 +713,10 @@ static int gemv_run(Ctx *c, GemvParams P, const W4Layout &L, int mode, int max_r
         if (want_quant_stage) return fail("w4a8 tile kernel: no quantising stage");
         if (P.pcap <= 0) return fail("w4a8 tile kernel: needs chunk-major activations");
         return tile_launch(c, P, grouped, L.bpg);
+    }
+    if (P.fold) {
+        if (want_quant_stage || P.tap || !P.xh) return fail("w4a8 fold kernel: needs fp16 activation rows, no taps");
+        return fold_launch(c, P, L);
     }
     if (gemv_uses_mma(max_rows)) {
         if (want_quant_stage) return fail("w4a8 gemv: quantising stage is not available beyond 2 rows per expert");
@@ -743,6 +797,15 @@ static int qrow_run(Ctx *c, const float *x, long long ldx, int K, const W4Layout
     if (grid_rows < 1) return 1;
     return launch(qrow_i8_kernel, dim3(grid_rows), dim3(256), 0, c->stream, "activation quantise launch", x, ldx, K,
                   L.kp, L.nblk, xq, sx, cs, n_rows_dev, n_rows, rowmap, pcap, amax_bits);
+}
+
+// Quantises rows for the fold kernel: fp16 copies of the int8 values, kp elements per row.
+static int qrow_f16_run(Ctx *c, const float *x, long long ldx, int K, const W4Layout &L, void *xh, float *sx,
+                        const int *n_rows_dev, int n_rows, int grid_rows, const unsigned *amax_bits = nullptr) {
+    if (grid_rows < 1) return 1;
+    const int vec = ((uintptr_t)x & 15) == 0 && (ldx & 3) == 0;
+    return launch(qrow_f16_kernel, dim3(grid_rows), dim3(256), 0, c->stream, "activation quantise launch", x, ldx, K, L.kp,
+                  (__half *)xh, sx, n_rows_dev, n_rows, amax_bits, vec);
 }
 
 // ------------------------------------------------------------- expert group
@@ -850,8 +913,8 @@ static int expert_group_impl(ColiCudaTensor *const *gates, ColiCudaTensor *const
     // grouped formats may pad K up to a multiple of gs: size for the largest gs (256)
     const size_t kpx = ((size_t)D + 255) / 256 * 256 + 256, kph = ((size_t)I + 255) / 256 * 256 + 256;
     if (!reserve(c, c->x, xb) || !reserve(c, c->y, xb) || !reserve(c, c->h, hb) ||
-        !reserve(c, c->xq, (size_t)total * kpx * 17 / 16 + 512) || !reserve(c, c->sx, (size_t)total * 4) ||
-        !reserve(c, c->xcs, (size_t)total * (kpx / 32) * 4) || !reserve(c, c->hq, (size_t)total * kph * 17 / 16 + 512) ||
+        !reserve(c, c->xq, (size_t)total * kpx * 2 + 512) || !reserve(c, c->sx, (size_t)total * 4) ||
+        !reserve(c, c->xcs, (size_t)total * (kpx / 32) * 4) || !reserve(c, c->hq, (size_t)total * kph * 2 + 512) ||
         !reserve(c, c->sh, (size_t)total * 4) || !reserve(c, c->hcs, (size_t)total * (kph / 32) * 4) ||
         !reserve(c, c->pin_x, xb, true) || !reserve(c, c->pin_y, xb, true))
         return 0;
@@ -873,7 +936,7 @@ static int expert_group_impl(ColiCudaTensor *const *gates, ColiCudaTensor *const
     struct ClassLaunch {
         int phase;  // 0: gate/up, 1: down
         const ColiCudaTensor *cls;
-        int cls_max, n;
+        int cls_max, n, rows;
         size_t off;  // byte offset of the region inside the block
     };
     std::vector<ClassLaunch> classes;
@@ -884,13 +947,14 @@ static int expert_group_impl(ColiCudaTensor *const *gates, ColiCudaTensor *const
         for (int lead = 0; lead < count; ++lead) {
             if (done[lead]) continue;
             const ColiCudaTensor *cls = lead_of[lead];
-            ClassLaunch cl{phase, cls, 0, 0, (blob.size() + 255) & ~(size_t)255};
+            ClassLaunch cl{phase, cls, 0, 0, 0, (blob.size() + 255) & ~(size_t)255};
             blob.resize(cl.off + 16);
             for (int j = lead; j < count; ++j) {
                 if (done[j] || !same_class(lead_of[j], cls)) continue;
                 done[j] = 1;
                 cl.cls_max = rows[j] > cl.cls_max ? rows[j] : cl.cls_max;
                 cl.n++;
+                cl.rows += rows[j];
                 const size_t at = blob.size();
                 if (cls->kind == 0) {
                     const F32Slot f = phase == 0 ? F32Slot{(const float *)gates[j]->data, (const float *)ups[j]->data,
@@ -933,9 +997,14 @@ static int expert_group_impl(ColiCudaTensor *const *gates, ColiCudaTensor *const
             continue;
         }
         const W4Layout &L = cl.cls->L;
-        ok = up ? qrow_run(c, (const float *)c->x.p, D, D, L, (int8_t *)c->xq.p, (float *)c->sx.p, (int *)c->xcs.p,
+        const bool fold = fold_pays(c, L, cl.phase, cl.cls_max, cl.rows, cl.n);
+        if (fold)
+            ok = up ? qrow_f16_run(c, (const float *)c->x.p, D, D, L, c->xq.p, (float *)c->sx.p, nullptr, total, total)
+                    : qrow_f16_run(c, (const float *)c->h.p, I, I, L, c->hq.p, (float *)c->sh.p, nullptr, total, total);
+        else
+            ok = up ? qrow_run(c, (const float *)c->x.p, D, D, L, (int8_t *)c->xq.p, (float *)c->sx.p, (int *)c->xcs.p,
                            nullptr, total, total, nullptr, gemv_uses_mma(cl.cls_max) ? total : 0)
-                : qrow_run(c, (const float *)c->h.p, I, I, L, (int8_t *)c->hq.p, (float *)c->sh.p, (int *)c->hcs.p,
+                    : qrow_run(c, (const float *)c->h.p, I, I, L, (int8_t *)c->hq.p, (float *)c->sh.p, (int *)c->hcs.p,
                            nullptr, total, total, nullptr, gemv_uses_mma(cl.cls_max) ? total : 0);
         GemvParams P{};
         P.slots = (const GemvSlot *)(region + 16);
@@ -946,6 +1015,9 @@ static int expert_group_impl(ColiCudaTensor *const *gates, ColiCudaTensor *const
         P.rowmap = nullptr;
         P.n_xrows = total;
         P.pcap = total;
+        P.fold = fold;
+        P.xh = up ? c->xq.p : c->hq.p;
+        P.xh_rows = total;
         P.out = (float *)(up ? c->h.p : c->y.p);
         P.out_stride = up ? I : D;
         ok = ok && gemv_run(c, P, L, up ? 0 : 1, cl.cls_max);

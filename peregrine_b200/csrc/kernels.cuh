@@ -90,8 +90,7 @@ constexpr int kXqChunkRowBytes = kChunkElems + 16;
 // int8 row (zero padded) and its scale it writes, per 32-element block,
 // -8 * sum(q): the term that turns the stream's stored nibbles (v+8) back into
 // signed weights inside the integer dot.  `rowmap` (optional) names the source row
-// of output row r; `pcap` > 0 selects the chunk-major layout with that row capacity, `pcap` < 0
-// the core-matrix layout of the tcgen05 kernel with capacity -pcap.
+// of output row r; `pcap` > 0 selects the chunk-major layout with that row capacity.
 __global__ void __launch_bounds__(256) qrow_i8_kernel(const float *__restrict__ x, long long ldx, int K, int kp,
                                                       int nblk, int8_t *__restrict__ xq, float *__restrict__ sx,
                                                       int *__restrict__ csum, const int *__restrict__ n_rows_dev,
@@ -139,13 +138,7 @@ __global__ void __launch_bounds__(256) qrow_i8_kernel(const float *__restrict__ 
         }
         int sum = q;
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (pcap < 0) {
-            // core-matrix order for the tcgen05 kernel: [chunk][16-element unit][row][16 bytes]
-            const long long cap = -pcap;
-            const int kk = (blk & 7) * 32 + lane;
-            xq[((((long long)(blk >> 3) * 16 + (kk >> 4)) * cap + row) << 4) + (kk & 15)] = (int8_t)q;
-            if (lane == 0) csum[((long long)(blk >> 3) * cap + row) * kChunkBlocks + (blk & 7)] = -8 * sum;
-        } else if (pcap > 0) {
+        if (pcap > 0) {
             const long long cr = (long long)(blk >> 3) * pcap + row;
             xq[cr * kXqChunkRowBytes + (blk & 7) * 32 + lane] = (int8_t)q;
             if (lane == 0) csum[cr * kChunkBlocks + (blk & 7)] = -8 * sum;
@@ -157,8 +150,7 @@ __global__ void __launch_bounds__(256) qrow_i8_kernel(const float *__restrict__ 
 }
 
 // Pair-ordered copy of already quantised token rows for the tensor-core kernels: output row p is
-// token pair_token[p], in the chunk-major layout (pcap > 0) or the core-matrix layout (pcap < 0)
-// described at qrow_i8_kernel.  Quantising once per token and copying int8 rows replaces
+// token pair_token[p], in the chunk-major layout described at qrow_i8_kernel.  Quantising once per token and copying int8 rows replaces
 // quantising every (token, expert) pair from fp32 again.  One CTA per pair row.
 __global__ void __launch_bounds__(256) gather_pair_rows_kernel(const int8_t *__restrict__ xq_tok,
                                                                const int *__restrict__ cs_tok,
@@ -170,19 +162,17 @@ __global__ void __launch_bounds__(256) gather_pair_rows_kernel(const int8_t *__r
     const int p = blockIdx.x;
     if (p >= *n_pairs_dev) return;
     const int tok = pair_token[p];
-    const long long cap = pcap < 0 ? -pcap : pcap;
     const uint4 *src = reinterpret_cast<const uint4 *>(xq_tok + (long long)tok * kp);
     for (int u = threadIdx.x; u < (kp >> 4); u += blockDim.x) {
         const int chunk = u >> 4, unit = u & 15;
-        const long long off = pcap < 0 ? ((((long long)chunk * 16 + unit) * cap + p) << 4)
-                                       : ((long long)chunk * cap + p) * kXqChunkRowBytes + unit * 16;
+        const long long off = ((long long)chunk * pcap + p) * kXqChunkRowBytes + unit * 16;
         *reinterpret_cast<uint4 *>(xqp + off) = __ldg(src + u);
     }
     const int nchunk = nblk >> 3;
     const int4 *csrc = reinterpret_cast<const int4 *>(cs_tok + (long long)tok * nblk);
     for (int u = threadIdx.x; u < 2 * nchunk; u += blockDim.x) {
         const int chunk = u >> 1;
-        *reinterpret_cast<int4 *>(csp + ((long long)chunk * cap + p) * kChunkBlocks + (u & 1) * 4) = __ldg(csrc + u);
+        *reinterpret_cast<int4 *>(csp + ((long long)chunk * pcap + p) * kChunkBlocks + (u & 1) * 4) = __ldg(csrc + u);
     }
     if (threadIdx.x == 0) sxp[p] = sx_tok[tok];
 }
@@ -279,8 +269,11 @@ struct GemvParams {
     int grid;  // host only: CTAs to launch (0 = one per SM)
     int pdl;   // host only: launch with programmatic stream serialisation (see griddep_wait)
     int tile_rb;  // host only: > 0 selects the large-batch tile kernel with this many row blocks in the grid
+    // host only: selects the fold kernel (kernels_fold.cuh); activations are the xh_rows fp16 rows of `xh`
+    bool fold;
+    const void *xh;
+    long long xh_rows;
     int blk_rpp;  // shared-row kernel: rows per work unit (32, 16 or 8); 0: chosen by the kernel
-    int umma;     // host only: with tile_rb > 0, take the tcgen05 kernel (activations in core-matrix order)
     const int *n_xrows_dev;     // rows actually valid (device scalar; nullptr: n_xrows)
     unsigned *amax_out;   // mode 0: per pair row, atomicMax of |h| bits (nullptr: off)
     float *out;
