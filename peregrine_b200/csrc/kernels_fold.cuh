@@ -649,7 +649,10 @@ __global__ void __launch_bounds__(kFoThreads, 1)
                 umma_commit(drain);
                 const long long t0 = clock64();
                 while (!mbar_try_wait(drain, 0u))
-                    if (clock64() - t0 > 2000000000LL) break;
+                    if (clock64() - t0 > 2000000000LL) {
+                        *fail = 1;
+                        break;
+                    }
             } else if (warp < 15) {
                 // ==================================================== weight chunks (and the work queue)
                 const int h = warp - 13;
@@ -744,10 +747,11 @@ __global__ void __launch_bounds__(kFoThreads, 1)
         __syncwarp();
     }
     // ---- common tail
-    if (*fail && tid == 0) report_error(P.err, kErrBarrierTimeout);
     __syncwarp();
     tmem_fence_before();
     __syncthreads();
+    // (behind the barrier: by now every role has noted its failure)
+    if (tid == 0 && *fail) report_error(P.err, kErrBarrierTimeout);
     if (warp == 12) {
         tmem_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
