@@ -662,28 +662,23 @@ static int fold_map_make(CUtensorMap *m, const void *base, long long rows, int k
         return fail("fold kernel: tensor map refused");
     return 1;
 }
-template <int TOK, bool GROUPED, int BPG>
+template <bool GROUPED, int BPG>
 static int fold_launch_t(Ctx *c, const GemvParams &P, const CUtensorMap &map) {
-    auto kfn = ffn_w4a8_fold_kernel<TOK, GROUPED, BPG>;
-    if (!ensure_smem(c, kfn, (size_t)fo_smem_bytes(TOK), "fold kernel shared-memory opt-in")) return 0;
-    return launch(kfn, dim3(c->sms), dim3(kFoThreads), (size_t)fo_smem_bytes(TOK), c->stream, "w4a8 fold kernel launch",
-                  map, P);
-}
-template <int TOK>
-static int fold_launch_g(Ctx *c, const GemvParams &P, const CUtensorMap &map, bool grouped, int bpg) {
-    if (!grouped) return fold_launch_t<TOK, false, 1>(c, P, map);
-    switch (bpg) {
-        case 1: return fold_launch_t<TOK, true, 1>(c, P, map);
-        case 2: return fold_launch_t<TOK, true, 2>(c, P, map);
-        case 4: return fold_launch_t<TOK, true, 4>(c, P, map);
-        case 8: return fold_launch_t<TOK, true, 8>(c, P, map);
-    }
-    return fail("w4a8 fold kernel: unsupported group size");
+    auto kfn = ffn_w4a8_fold_kernel<GROUPED, BPG>;
+    if (!ensure_smem(c, kfn, (size_t)kFoSmemBytes, "fold kernel shared-memory opt-in")) return 0;
+    return launch(kfn, dim3(c->sms), dim3(kFoThreads), (size_t)kFoSmemBytes, c->stream, "w4a8 fold kernel launch", map, P);
 }
 static int fold_launch(Ctx *c, const GemvParams &P, const W4Layout &L) {
     CUtensorMap map;
     if (!fold_map_make(&map, P.xh, P.xh_rows, L.kp)) return 0;
-    return fold_launch_g<kFoTok>(c, P, map, L.grouped != 0, L.bpg);
+    if (!L.grouped) return fold_launch_t<false, 1>(c, P, map);
+    switch (L.bpg) {
+        case 1: return fold_launch_t<true, 1>(c, P, map);
+        case 2: return fold_launch_t<true, 2>(c, P, map);
+        case 4: return fold_launch_t<true, 4>(c, P, map);
+        case 8: return fold_launch_t<true, 8>(c, P, map);
+    }
+    return fail("w4a8 fold kernel: unsupported group size");
 }
 
 // Fills the layout-dependent fields and launches.  `max_rows` bounds the rows of any slot:

@@ -18,14 +18,14 @@
 //     memory, whose bandwidth the B operand and the copies need.
 //
 // Tile of a CTA: 2 halves of 128 weight rows (mode 0: 128 gate + the same 128 up rows, so a thread holds
-// both values of its SwiGLU; mode 1: 256 down rows) x TOK activation rows of one expert.  Roles:
+// both values of its SwiGLU; mode 1: 256 down rows) x 64 activation rows of one expert.  Roles:
 //
 //   warps 0-7    fold and epilogue: warp w owns TMEM lanes 32 (w % 4).. and the 16-column groups
 //                w/4, w/4 + 2, ..; accumulators in registers
 //   warps 8-11   expand: 32 rows of both halves per warp, one 32-element block at a time, into a ring of
 //                four blocks in tensor memory
 //   warp 12      one lane issues the MMAs: four per block (two halves, K = 16 each); dots of a group go to
-//                one of NBUF accumulators of TOK columns
+//                one of six accumulators of 64 columns
 //   warps 13, 14 bulk copies of the packed weight chunks (8 tiles each; issuing one costs ~130 cycles), a
 //                chunk of 256 elements per stage; warp 13 also takes work items from a device counter and
 //                publishes them to the other roles
@@ -56,14 +56,14 @@ constexpr int kFoAStages = 4;       // 32-element blocks of expanded weights in 
 constexpr int kFoACol = 384;        // their first column: 4 blocks x 2 halves x 16 columns
 constexpr int kFoQueue = 4;
 
-__host__ __device__ constexpr int fo_wstages(int tok) { return tok == 128 ? 2 : (tok == 64 ? 3 : 4); }
-__host__ __device__ constexpr int fo_nbuf(int tok) { return tok == 128 ? 3 : (tok == 64 ? 6 : 8); }
-__host__ __device__ constexpr int fo_woff(int tok) { return kFoXStages * tok * 128; }
-__host__ __device__ constexpr int fo_tab_off(int tok) { return fo_woff(tok) + fo_wstages(tok) * kFoWStageBytes; }
+constexpr int kFoWStages = 3;        // chunks of the item's 16 tiles
+constexpr int kFoNBuf = 6;           // accumulators of kFoTok columns in tensor memory
+constexpr int kFoWOff = kFoXStages * kFoTok * 128;
+constexpr int kFoTabOff = kFoWOff + kFoWStages * kFoWStageBytes;
 constexpr int kFoTabBytes = (3 * kFoMaxSlots + 4) * 4;
-__host__ __device__ constexpr int fo_bar_off(int tok) { return fo_tab_off(tok) + kFoTabBytes; }
+constexpr int kFoBarOff = kFoTabOff + kFoTabBytes;
 // 1024 bytes of slack: the swizzled tiles need a 1024-byte boundary
-__host__ __device__ constexpr int fo_smem_bytes(int tok) { return fo_bar_off(tok) + 512 + 1024; }
+constexpr int kFoSmemBytes = kFoBarOff + 512 + 1024;
 
 // Work counter of the launches (next item, CTAs that have finished; the last one clears both): launches
 // on a device are ordered by the context's stream.  Zero when the module is loaded.
@@ -262,12 +262,12 @@ struct RingPos {
 
 // Grid: one CTA per SM.  Activations: fp16 rows through `xmap` (qrow_f16_kernel / gather_pair_f16_kernel),
 // P.sx per row; P.xq / P.csum are not used.
-template <int TOK, bool GROUPED, int BPG>
+template <bool GROUPED, int BPG>
 __global__ void __launch_bounds__(kFoThreads, 1)
     ffn_w4a8_fold_kernel(const __grid_constant__ CUtensorMap xmap, const GemvParams P) {
     constexpr int GPC = kChunkBlocks / BPG;
     constexpr int CHUNK_BYTES = kChunkSlabBytes + (GROUPED ? GPC * 64 : 0);
-    constexpr int WST = fo_wstages(TOK), NBUF = fo_nbuf(TOK), NI = TOK / 32;
+    constexpr int TOK = kFoTok, WST = kFoWStages, NBUF = kFoNBuf;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ int s_fail, s_total;
@@ -275,12 +275,12 @@ __global__ void __launch_bounds__(kFoThreads, 1)
     __shared__ __align__(16) int4 s_queue[kFoQueue];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t smem_u = smem_u32(smem);
-    const uint32_t bar0 = smem_u + fo_bar_off(TOK);
+    const uint32_t bar0 = smem_u + kFoBarOff;
     const uint32_t xfull = bar0, xempty = xfull + 8 * kFoXStages, wfull = xempty + 8 * kFoXStages,
                    wempty = wfull + 8 * 4, afull = wempty + 8 * 4, aempty = afull + 8 * kFoAStages,
                    dfull = aempty + 8 * kFoAStages, dempty = dfull + 8 * 8, qfull = dempty + 8 * 8,
                    qempty = qfull + 8 * kFoQueue, drain = qempty + 8 * kFoQueue;
-    int *t_key = reinterpret_cast<int *>(smem + fo_tab_off(TOK));  // rows per block of a slot
+    int *t_key = reinterpret_cast<int *>(smem + kFoTabOff);  // rows per block of a slot
     int *t_slot = t_key + kFoMaxSlots;                              // slot of rank r
     int *t_cum = t_slot + kFoMaxSlots;                              // first row block of rank r
     volatile int *fail = &s_fail;
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kFoThreads, 1)
 #pragma unroll 1
                 for (int chunk = 0; GROUPED && chunk < P.nchunk; ++chunk) {
                     um_spin(wfull + 8 * wp.i, wp.ph, fail);
-                    const uint8_t *st = smem + fo_woff(TOK) + wp.i * kFoWStageBytes;
+                    const uint8_t *st = smem + kFoWOff + wp.i * kFoWStageBytes;
                     constexpr int SB = GPC < 2 ? 1 : 2;  // groups whose scales are read at once
                     // (one or two groups per loop trip: the body has to stay inside the instruction cache)
 #pragma unroll 1
@@ -525,16 +525,10 @@ __global__ void __launch_bounds__(kFoThreads, 1)
                             for (int c = 0; c < 8; ++c) acc[h][k][c] = acc[h][k + 1][c];
                 }
             };
-            if constexpr (NI == 4) {
-                if (cnt >= 4)
-                    run_item(std::integral_constant<int, 4>{});
-                else if (cnt == 3)
-                    run_item(std::integral_constant<int, 3>{});
-            }
-            if constexpr (NI >= 2) {
-                if (cnt == 2) run_item(std::integral_constant<int, 2>{});
-            }
-            if (cnt <= 1) run_item(std::integral_constant<int, 1>{});
+            if (cnt == 2)
+                run_item(std::integral_constant<int, 2>{});
+            else
+                run_item(std::integral_constant<int, 1>{});
             ok = __all_sync(0xffffffffu, !*fail);
         }
     } else if (warp < 12) {
@@ -551,7 +545,7 @@ __global__ void __launch_bounds__(kFoThreads, 1)
             for (int chunk = 0; chunk < P.nchunk && ok; ++chunk) {
                 ok = __all_sync(0xffffffffu, um_wait(wfull + 8 * wp.i, wp.ph, fail));
                 if (!ok) break;
-                const uint8_t *st = smem + fo_woff(TOK) + wp.i * kFoWStageBytes + off;
+                const uint8_t *st = smem + kFoWOff + wp.i * kFoWStageBytes + off;
                 uint4 w0 = *reinterpret_cast<const uint4 *>(st);
                 uint4 w1 = *reinterpret_cast<const uint4 *>(st + 8 * kChunkMaxBytes);
 #pragma unroll 1
@@ -693,7 +687,7 @@ __global__ void __launch_bounds__(kFoThreads, 1)
                         ok = um_wait(wempty + 8 * wp.i, wp.ph ^ 1u, fail);
                         if (!ok) break;
                         const uint32_t bar = wfull + 8 * wp.i;
-                        const uint32_t dst = smem_u + fo_woff(TOK) + wp.i * kFoWStageBytes + 8 * h * kChunkMaxBytes;
+                        const uint32_t dst = smem_u + kFoWOff + wp.i * kFoWStageBytes + 8 * h * kChunkMaxBytes;
                         // (the phase needs both warps' arrivals, so no copy can complete it early)
                         mbar_expect_tx(bar, n_wt * CHUNK_BYTES);
                         if (n_wt == 8) {
