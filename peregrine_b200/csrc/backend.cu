@@ -591,6 +591,13 @@ static size_t act_xq_bytes(const W4Layout &L, size_t rows, int max_rows) {
     return gemv_uses_mma(max_rows) ? (size_t)L.nchunk * rows * kXqChunkRowBytes : rows * (size_t)L.kp;
 }
 
+// Scratch for them that also holds the fold kernel's rows (2 bytes per element against 17/16), whichever kernel
+// the call takes.  Recorded graphs keep the addresses of a context's scratch, which moves when a call needs more
+// than any before it: that has to depend on the call's rows and widths alone, not on the kernel it is given.
+static size_t act_scratch_bytes(const W4Layout &L, size_t rows, int max_rows) {
+    return act_xq_bytes(L, rows, max_rows) * 32 / 17;
+}
+
 // True when the launch's activation rows fit in shared memory beside the rings of the dp4a kernel.
 static bool gemv_rows_fit(Ctx *c, int n_xrows, const W4Layout &L) {
     return (size_t)kRingBytes + kGemvBarBytes + gemv_xs_bytes(n_xrows, L.kp, L.nblk) + 1024 <= c->smem_optin;

@@ -1,0 +1,72 @@
+"""Calls whose expert kernel is the tcgen05 fold kernel, bit for bit against the CPU oracle: single matrices,
+expert groups, layers and wide shared experts, at the edges of its tiles and of the rules that choose it."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle as po
+from peregrine_b200 import cuda
+from peregrine_b200.synth import synth_matrix
+from tests.gpu_common import bits
+
+pytestmark = pytest.mark.gpu
+
+
+def upload(dev, m):
+    return (cuda.Tensor.upload_grouped(dev, m.q, m.scale, m.i_n, m.o_n, m.gs) if m.gs
+            else cuda.Tensor.upload(dev, m.q, m.scale, 2, m.i_n, m.o_n))
+
+
+def apply(m, x):
+    return po.Weight(m.q, m.scale, 4 if m.gs else 2, m.gs, m.i_n, m.o_n).apply(x, x.shape[0])
+
+
+class DevRows:
+    def __init__(self, dev, rows, width):
+        self.dev, self.shape = dev, (rows, width)
+        self.ptr = cuda.lib().coli_cuda_pipe_alloc(dev, rows * width * 4)
+        assert self.ptr
+
+    def put(self, a):
+        a = np.ascontiguousarray(a, np.float32)
+        assert cuda.lib().coli_cuda_pipe_upload(self.dev, self.ptr, a.ctypes.data, a.nbytes) == 1
+
+    def get(self, rows=None):
+        out = np.empty((self.shape[0] if rows is None else rows, self.shape[1]), np.float32)
+        assert cuda.lib().coli_cuda_pipe_download(self.dev, self.ptr, out.ctypes.data, out.nbytes) == 1
+        return out
+
+    def free(self):
+        cuda.lib().coli_cuda_pipe_free(self.dev, self.ptr)
+
+
+def gemm(t, y, x, rows):
+    return cuda.lib().coli_cuda_pipe_gemm(t.handle, C.c_void_p(y.ptr), C.c_void_p(x.ptr), rows)
+
+
+def test_scratch_depends_on_rows_and_width_not_on_the_kernel(dev):
+    """A call that has sized the scratch for its rows and width has sized it for every matrix of that width: the
+    product of a taller one, which the fold kernel takes, is recorded without a call of its own before (growing
+    scratch would end the recording), and the replay gives the oracle's rows.  The row count is above all others
+    of the suite, so that no earlier test has left more scratch behind."""
+    lib = cuda.lib()
+    rng = np.random.default_rng(61)
+    k, rows = 2048, 5000
+    small, tall = synth_matrix(rng, 200, k, 32), synth_matrix(rng, 600, k, 32)
+    ts, tt = upload(dev, small), upload(dev, tall)
+    x, y = DevRows(dev, rows, k), DevRows(dev, rows, 600)
+    xh = rng.standard_normal((rows, k)).astype(np.float32)
+    x.put(xh)
+    assert gemm(ts, y, x, rows) == 1 and lib.coli_cuda_pipe_sync(dev) == 1
+    assert lib.coli_cuda_graph_begin(dev) == 1
+    rc = gemm(tt, y, x, rows)
+    g = C.c_void_p()
+    assert lib.coli_cuda_graph_end(dev, C.byref(g)) == 1 and rc == 1
+    assert lib.coli_cuda_graph_launch(g) == 1
+    pick = np.r_[0:40, 2480:2520, rows - 40:rows]
+    assert np.array_equal(bits(y.get()[pick]), bits(apply(tall, xh[pick])))
+    assert cuda.last_device_error(dev) == 0
+    lib.coli_cuda_graph_free(g)
+    for b in (x, y, ts, tt):
+        b.free()
