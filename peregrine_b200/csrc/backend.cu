@@ -2,7 +2,6 @@
 // calls of the reference ABI and the device-resident MoE layer.  Declarations
 // and the reference lines each entry point replaces are in
 // include/peregrine_b200.h.
-#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -627,22 +626,6 @@ static int tile_launch(Ctx *c, const GemvParams &P, bool grouped, int bpg) {
 }
 
 // ---- fold kernel (tcgen05)
-// Can it hold the launch at all: its slot table, and for per-row scales the whole row's integer dot, which
-// has to stay exact in the fp32 accumulator (8 * 128 * K <= 2^24).
-static bool fold_fits(const W4Layout &L, int slots_max) {
-    return slots_max <= kFoMaxSlots && (L.grouped || L.kp <= 16384);
-}
-// Is it the faster one for `slots` experts with `rows` rows together and at most `max_rows` each?  Its items are
-// long pipelines (256 weight rows, all of K): it needs K of 8 chunks (measured at 301 tokens: 6 chunks 173 us
-// against 160 for the tile kernel, 8 chunks 160 against 170 at 128 tokens) and items for most of the CTAs
-// (one 2048 x 8192 matrix at 100 rows: 64 items, 44 us against 40 for the small-batch kernel; 6144 x 12288:
-// 96 items, 69 against 94), and below 32 rows most of its columns are padding (6144 x 32000, 12 rows: 86 us
-// against 72; 32 rows: 86 against 93; 64 rows: 100 against 147).
-static bool fold_pays(Ctx *c, const W4Layout &L, int mode, int max_rows, long long rows, int slots) {
-    const long long n_ob = mode == 0 ? (L.ntile + 7) / 8 : (L.ntile + 15) / 16;
-    const long long units = std::max<long long>(slots, (rows + kFoTok - 1) / kFoTok);
-    return fold_fits(L, slots) && L.nchunk >= 8 && max_rows >= 32 && rows >= 16LL * slots && 5 * n_ob * units >= 3LL * c->sms;
-}
 static size_t act_f16_bytes(const W4Layout &L, size_t rows) { return rows * (size_t)L.kp * 2; }
 
 // fp16 activation rows [rows][kp] as boxes of 64 elements x 32 rows, 128-byte swizzle.
@@ -938,7 +921,8 @@ static int expert_group_impl(ColiCudaTensor *const *gates, ColiCudaTensor *const
     struct ClassLaunch {
         int phase;  // 0: gate/up, 1: down
         const ColiCudaTensor *cls;
-        int cls_max, n, rows;
+        int cls_max, n;
+        RowBlocks blocks;
         size_t off;  // byte offset of the region inside the block
     };
     std::vector<ClassLaunch> classes;
@@ -949,14 +933,14 @@ static int expert_group_impl(ColiCudaTensor *const *gates, ColiCudaTensor *const
         for (int lead = 0; lead < count; ++lead) {
             if (done[lead]) continue;
             const ColiCudaTensor *cls = lead_of[lead];
-            ClassLaunch cl{phase, cls, 0, 0, 0, (blob.size() + 255) & ~(size_t)255};
+            ClassLaunch cl{phase, cls, 0, 0, {}, (blob.size() + 255) & ~(size_t)255};
             blob.resize(cl.off + 16);
             for (int j = lead; j < count; ++j) {
                 if (done[j] || !same_class(lead_of[j], cls)) continue;
                 done[j] = 1;
                 cl.cls_max = rows[j] > cl.cls_max ? rows[j] : cl.cls_max;
                 cl.n++;
-                cl.rows += rows[j];
+                cl.blocks.add(rows[j]);
                 const size_t at = blob.size();
                 if (cls->kind == 0) {
                     const F32Slot f = phase == 0 ? F32Slot{(const float *)gates[j]->data, (const float *)ups[j]->data,
@@ -999,7 +983,7 @@ static int expert_group_impl(ColiCudaTensor *const *gates, ColiCudaTensor *const
             continue;
         }
         const W4Layout &L = cl.cls->L;
-        const bool fold = fold_pays(c, L, cl.phase, cl.cls_max, cl.rows, cl.n);
+        const bool fold = fold_beats_block(L, cl.phase, cl.blocks, c->sms);
         if (fold)
             ok = up ? qrow_f16_run(c, (const float *)c->x.p, D, D, L, c->xq.p, (float *)c->sx.p, nullptr, total, total)
                     : qrow_f16_run(c, (const float *)c->h.p, I, I, L, c->hq.p, (float *)c->sh.p, nullptr, total, total);

@@ -1,0 +1,71 @@
+// Which expert kernel a large launch is given: rules on sizes and weight format, plain host code that the CPU
+// tests compile too.
+#pragma once
+#include "w4_layout.h"
+
+namespace pgb {
+
+constexpr int kFoTok = 64;         // activation rows of a fold-kernel item
+constexpr int kFoMaxSlots = 1024;  // slots of its launches
+
+// Can the fold kernel hold the launch at all: its slot table, and for per-row scales the whole row's integer dot,
+// which has to stay exact in the fp32 accumulator (8 * 128 * K <= 2^24).
+inline bool fold_fits(const W4Layout &L, int slots_max) {
+    return slots_max <= kFoMaxSlots && (L.grouped || L.kp <= 16384);
+}
+
+// The rows of a launch whose slots the host knows, as the two kernels cut them.
+struct RowBlocks {
+    int slots = 0, max_rows = 0;
+    long long narrow = 0, wide = 0;           // fold kernel: row blocks of at most 32 and of up to 64 rows
+    long long units[5] = {0, 0, 0, 0, 0};     // small-batch kernel: units of 8, 16, 24 and 32 rows
+    void add(int rows) {
+        if (rows < 1) return;
+        ++slots;
+        max_rows = rows > max_rows ? rows : max_rows;
+        cut(rows, kFoTok, [this](int r, long long n) { (r <= 32 ? narrow : wide) += n; });
+        cut(rows, 32, [this](int r, long long n) { units[(r + 7) / 8] += n; });
+    }
+
+  private:
+    template <typename F>
+    static void cut(int rows, int most, F use) {  // even blocks of whole groups of 8 rows
+        const int blocks = (rows + most - 1) / most, per = 8 * (((rows + 7) / 8 + blocks - 1) / blocks);
+        use(per < rows ? per : rows, rows / per > 0 ? rows / per : 1);
+        if (rows > per && rows % per) use(rows % per, 1);
+    }
+};
+
+// Is the fold kernel faster than the shared-row small-batch kernel for these rows?  Both are given the time of
+// their rounds of items over the SMs.  The constants (us) are fitted to measured launches (B200; one matrix of K
+// 1536..6144, O 2048..33000 and 24..1200 rows, both phases of groups of 1..40 experts with up to 150 rows, five
+// formats).  Over the 1890 of them with 8+ chunks and 32+ rows the choice is 0.3 % behind the faster kernel of
+// each; 11 lose over 2 %, at most 12 %.
+//   * fold: an item is 256 weight rows x up to 64 rows and always costs its whole width (or half of it); a last
+//     round that few items fill costs like a full one.  6144 x 16000, group 32: 128 rows 144 -> 97 us, 129 rows
+//     (three blocks of 43, 189 items) 145 against 170.
+//   * small batch: units of 32 rows whose cost goes with their groups of 8 rows; cut finer when items are few.
+//     2048 x 4096, 64 rows: 28 us against 44.
+// Below 8 chunks of K and below 32 rows the small-batch kernel stays: nothing was settled there.
+inline bool fold_beats_block(const W4Layout &L, int mode, const RowBlocks &R, int sms) {
+    if (!fold_fits(L, R.slots) || L.nchunk < 8 || R.max_rows < 32) return false;
+    struct Cost {
+        double fold, narrow, block;  // us per chunk and round; narrow items relative to wide ones
+    };
+    const Cost per_row{1.80, 1.00, 2.15};
+    const Cost by_bpg[4] = {{3.20, 0.75, 2.25}, {2.60, 0.85, 2.05}, {2.15, 0.90, 2.05}, {1.90, 1.00, 2.05}};
+    const Cost &c = !L.grouped ? per_row : by_bpg[L.bpg == 1 ? 0 : L.bpg == 2 ? 1 : L.bpg == 4 ? 2 : 3];
+    const double n_ob = mode == 0 ? (L.ntile + 7) / 8 : (L.ntile + 15) / 16;
+    const double chunks = L.nchunk + (mode == 0 ? 1.0 : 0.5);  // the epilogue, in chunks
+    const double items = n_ob * (R.narrow + R.wide), work = n_ob * (R.narrow * c.narrow + R.wide);
+    const double fold_rounds = items > sms ? work / sms + 0.4 * work / items : (R.wide ? 1.0 : c.narrow);
+    double units = 0, weight = 0;
+    for (int g = 1; g <= 4; ++g) {
+        units += n_ob * R.units[g];
+        weight += n_ob * R.units[g] * (0.28 + 0.18 * g);
+    }
+    const double block_rounds = weight / sms + (units > sms ? 0.5 : 0.42);
+    return 18.0 + c.fold * chunks * fold_rounds < 14.0 + c.block * chunks * block_rounds;
+}
+
+}  // namespace pgb

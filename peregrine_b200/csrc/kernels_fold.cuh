@@ -41,13 +41,12 @@
 
 #include <type_traits>
 
+#include "expert_route.h"
 #include "kernels_tcgen05.cuh"
 
 namespace pgb {
 
-constexpr int kFoTok = 64;          // activation rows of a tile
 constexpr int kFoThreads = 512;
-constexpr int kFoMaxSlots = 1024;   // slots of a launch
 constexpr int kFoXGroup = 64;       // elements of K per activation copy (one 128-byte swizzle row of fp16)
 constexpr int kFoXStages = 8;
 constexpr int kFoXBoxRows = 32;

@@ -15,7 +15,7 @@ def build_hostcheck(force: bool = False) -> str:
     """Host-only helper library of the CPU tests: the tile-stream walk compiled from the same
     layout header and repacker the CUDA backend uses."""
     srcs = [os.path.join(HERE, "w4_hostcheck.cpp"), os.path.join(CSRC, "w4_host.cpp")]
-    deps = srcs + [os.path.join(CSRC, "w4_layout.h"), os.path.join(CSRC, "w4_host.h")]
+    deps = srcs + [os.path.join(CSRC, h) for h in ("w4_layout.h", "w4_host.h", "expert_route.h")]
     stale = force or not os.path.exists(HOSTCHECK) or any(
         os.path.getmtime(p) > os.path.getmtime(HOSTCHECK) for p in deps)
     if stale:
@@ -37,6 +37,9 @@ def lib():
         L.pgb_hc_qrow.argtypes = [vp, i, i, i, vp, vp, vp]
         L.pgb_hc_qrow.restype = None
         L.pgb_hc_walk.argtypes = [vp, vp, i, i, i, i, vp, vp, vp, i, vp, vp]
+        L.pgb_hc_fold_beats_block.argtypes = [i, i, i, i, vp, i, i]
+        L.pgb_hc_row_blocks.argtypes = [i, vp]
+        L.pgb_hc_row_blocks.restype = None
         _lib = L
     return _lib
 
@@ -87,3 +90,18 @@ def walk(stream, rs, L, xq, cs, sx, nrows, want_tap=False):
                              cs.ctypes.data, sx.ctypes.data, nrows, y.ctypes.data,
                              None if tap is None else tap.ctypes.data)
     return (y, tap) if want_tap else y
+
+
+SMS = 148  # multiprocessors of a B200
+
+
+def fold_beats_block(o, k, gs, mode, rows):
+    """Does a launch of these rows per slot go to the fold kernel (mode 0: gate/up, 1: one matrix)?"""
+    r = np.ascontiguousarray(np.atleast_1d(rows), np.int32)
+    return lib().pgb_hc_fold_beats_block(o, k, gs, mode, r.ctypes.data, r.size, SMS) == 1
+
+
+def row_blocks(rows):
+    out = np.zeros(6, np.int64)
+    lib().pgb_hc_row_blocks(rows, out.ctypes.data)
+    return [int(v) for v in out]

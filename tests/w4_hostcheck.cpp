@@ -7,6 +7,7 @@
 #include <cstring>
 #include <vector>
 
+#include "expert_route.h"
 #include "w4_host.h"
 
 using namespace pgb;
@@ -129,4 +130,21 @@ HC_API int pgb_hc_walk(const uint8_t *stream, const float *row_scales, int O, in
         }
     }
     return 1;
+}
+
+// The kernel choice of a launch whose rows per slot are known: 1 = fold kernel, 0 = small-batch kernels.
+HC_API int pgb_hc_fold_beats_block(int O, int K, int gs, int mode, const int *rows, int n, int sms) {
+    W4Layout L;
+    if (!w4_layout_make(&L, O, K, gs != 0, gs)) return -1;
+    RowBlocks R;
+    for (int i = 0; i < n; ++i) R.add(rows[i]);
+    return fold_beats_block(L, mode, R, sms) ? 1 : 0;
+}
+// How that choice cuts a slot's rows: {fold blocks <= 32 rows, fold blocks, units of 8, 16, 24, 32 rows}.
+HC_API void pgb_hc_row_blocks(int rows, long long *out6) {
+    RowBlocks R;
+    R.add(rows);
+    out6[0] = R.narrow;
+    out6[1] = R.narrow + R.wide;
+    for (int g = 1; g <= 4; ++g) out6[1 + g] = R.units[g];
 }
