@@ -7,8 +7,11 @@ import pytest
 
 import oracle as po
 from peregrine_b200 import cuda
-from peregrine_b200.synth import synth_matrix
+from peregrine_b200.resident import upload_layer
+from peregrine_b200.synth import synth_expert, synth_layer, synth_matrix, synth_tokens
+from tests import hostcheck as hc
 from tests.gpu_common import bits
+from tests.refmodel import oracle_layer_forward
 
 pytestmark = pytest.mark.gpu
 
@@ -41,6 +44,20 @@ class DevRows:
         cuda.lib().coli_cuda_pipe_free(self.dev, self.ptr)
 
 
+def fold_launches(dev, call):
+    """Runs `call` and returns its result and how many of its launches were the fold kernel's (None where the
+    profiler records no kernels)."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        out = call()
+        assert cuda.lib().coli_cuda_pipe_sync(dev) == 1
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "kernel" in e.name]
+    return out, sum("ffn_w4a8_fold_kernel" in n for n in names) if names else None
+
+
 def gemm(t, y, x, rows):
     return cuda.lib().coli_cuda_pipe_gemm(t.handle, C.c_void_p(y.ptr), C.c_void_p(x.ptr), rows)
 
@@ -70,3 +87,29 @@ def test_scratch_depends_on_rows_and_width_not_on_the_kernel(dev):
     lib.coli_cuda_graph_free(g)
     for b in (x, y, ts, tt):
         b.free()
+
+
+@pytest.mark.parametrize("m,want_fold", [(300, 1), (650, 2)])
+def test_wide_shared_expert_chooses_per_phase(dev, m, want_fold):
+    """A shared expert of its own width: 300 tokens fill the SMs with gate/up items (20 weight blocks) but not
+    with down items (8), 650 tokens with both."""
+    hidden, wide = 2048, 2560
+    assert hc.fold_beats_block(wide, hidden, 32, 0, m)
+    assert hc.fold_beats_block(hidden, wide, 32, 1, m) == (want_fold == 2)
+    layer = synth_layer(31, hidden=hidden, inter=256, n_experts=24, k=1, gs=32, distinct_experts=2)
+    layer.shared = synth_expert(np.random.default_rng(310), hidden, wide, 32)
+    ml = upload_layer(dev, layer)
+    x = synth_tokens(32, m, hidden)
+    out = np.empty_like(x)
+    ml.forward(x, out)  # sizes the scratch
+    got, n = fold_launches(dev, lambda: ml.forward(x, out))
+    if n is not None:
+        assert n == want_fold + routed_folds(layer, m)
+    assert np.array_equal(bits(got), bits(oracle_layer_forward(layer, x, threads=8)))
+    assert cuda.last_device_error(dev) == 0
+    ml.free()
+
+
+def routed_folds(layer, m):
+    """Launches of the routed experts that go to the fold kernel."""
+    return 2 if layer.hidden >= 2048 and m >= 48 and 2 * m * layer.k >= 3 * layer.n_experts else 0
