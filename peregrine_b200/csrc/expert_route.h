@@ -1,6 +1,8 @@
 // Which expert kernel a large launch is given: rules on sizes and weight format, plain host code that the CPU
 // tests compile too.
 #pragma once
+#include <cmath>
+
 #include "w4_layout.h"
 
 namespace pgb {
@@ -66,6 +68,44 @@ inline bool fold_beats_block(const W4Layout &L, int mode, const RowBlocks &R, in
     }
     const double block_rounds = weight / sms + (units > sms ? 0.5 : 0.42);
     return 18.0 + c.fold * chunks * fold_rounds < 14.0 + c.block * chunks * block_rounds;
+}
+
+// The same against the CTA-tiled mma.sync kernel, for one phase of a layer of M tokens, top-k of E experts, whose rows
+// per expert only the device knows: an even spread is assumed.  Items come in rounds over the SMs; the fold kernel
+// needs a full round or more, and enough chunks in all for its long pipelines to pay for their start.  Measured at
+// 13 shapes x 5 formats x 48..4000 tokens (gate/up and down separately, us tiles -> fold): gate/up of 24 chunks
+// group 32 3252 -> 2988, of 8 chunks 371 -> 380 at 2000 tokens and 80 -> 67 at 128; down of 8 chunks 1787 -> 1520,
+// of 4 chunks 205 -> 192; where items are few (768 x 2048, 16 experts, 48 tokens: 102 items) 34 -> 50.  Per-row
+// scales, without a fold per group, are ahead from one round on (1600 x 2560, 8 experts, 200 tokens: 53 -> 47).  Below 8 chunks
+// gate/up, whose epilogue is the longer one, stays with the tiles (6 chunks group 64: 137 -> 146); grouped down of
+// one chunk too (58 -> 63).  Over all 611 layers the choice is 5.7 % ahead of the tiles alone and 0.4 % behind the
+// better kernel of each phase; 6 of them lose over 2 %, at most 8 %.
+// (More tokens never take a layer back to the tiles: its scratch is sized by the most tokens it has seen.)
+inline bool fold_beats_tiles(const W4Layout &L, int mode, int M, int E, int k, int sms) {
+    if (!fold_fits(L, E + 1) || L.nchunk < (mode == 0 ? 8 : L.grouped ? 2 : 1)) return false;
+    const double n_ob = mode == 0 ? (L.ntile + 7) / 8 : (L.ntile + 15) / 16;
+    const double touched = E * (1.0 - std::pow(1.0 - (double)(k < E ? k : E) / E, M));
+    const double full = (double)M * k / kFoTok;
+    const double rounds = n_ob * ((touched > full ? touched : full) + (M + kFoTok - 1) / kFoTok) / sms;
+    if (!L.grouped) return rounds >= 1.0 && rounds * L.nchunk >= (mode == 0 ? 8.0 : 6.0);
+    return rounds >= 1.5 && rounds * L.nchunk >= (mode == 0 ? 24.0 : 8.0);
+}
+
+// The expert kernels of a layer call of 3 or more tokens.  Batches of 48+ tokens with on average 1.5+ rows per routed
+// expert (measured crossover between 32 and 64 tokens at 256 experts top-8: 255 us against 378, 575 against 477)
+// leave the small-batch kernels.  `want` (-1: none) forces a choice: 0 small batch, 1 tiles, 2 fold kernel.
+struct LayerRoute {
+    bool tiles_gu, tiles_dn, fold_gu, fold_dn;
+};
+inline LayerRoute layer_route(const W4Layout &Lgu, const W4Layout &Ldn, int M, int E, int k, int sms, int want) {
+    LayerRoute r{};
+    const bool large = want < 0 ? M >= 48 && 2LL * M * k >= 3LL * E : want > 0;
+    if (!large) return r;
+    r.fold_gu = want == 2 ? fold_fits(Lgu, E + 1) : want < 0 && fold_beats_tiles(Lgu, 0, M, E, k, sms);
+    r.fold_dn = want == 2 ? fold_fits(Ldn, E + 1) : want < 0 && fold_beats_tiles(Ldn, 1, M, E, k, sms);
+    r.tiles_gu = !r.fold_gu;
+    r.tiles_dn = !r.fold_dn;
+    return r;
 }
 
 }  // namespace pgb

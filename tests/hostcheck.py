@@ -38,6 +38,7 @@ def lib():
         L.pgb_hc_qrow.restype = None
         L.pgb_hc_walk.argtypes = [vp, vp, i, i, i, i, vp, vp, vp, i, vp, vp]
         L.pgb_hc_fold_beats_block.argtypes = [i, i, i, i, vp, i, i]
+        L.pgb_hc_layer_route.argtypes = [i] * 8
         L.pgb_hc_row_blocks.argtypes = [i, vp]
         L.pgb_hc_row_blocks.restype = None
         _lib = L
@@ -105,3 +106,9 @@ def row_blocks(rows):
     out = np.zeros(6, np.int64)
     lib().pgb_hc_row_blocks(rows, out.ctypes.data)
     return [int(v) for v in out]
+
+
+def layer_route(hidden, inter, gs, m, experts, k, want=-1):
+    """(gate/up, down) of a layer call: "small", "tiles" or "fold"."""
+    r = lib().pgb_hc_layer_route(hidden, inter, gs, m, experts, k, SMS, want)
+    return tuple("fold" if r >> p & 1 else "tiles" if r >> (2 + p) & 1 else "small" for p in (0, 1))

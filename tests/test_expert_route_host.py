@@ -44,3 +44,46 @@ def test_what_the_fold_kernel_is_not_given():
     assert hc.fold_beats_block(33000, 16384, 0, 1, 1000)
     assert not hc.fold_beats_block(33000, 16385, 0, 1, 1000)      # per-row dots beyond the accumulator's 24 bits
     assert hc.fold_beats_block(33000, 16385, 32, 1, 1000)         # (a group's dot stays far below)
+
+
+FULL, SMALL = (6144, 2048, 256, 8), (2048, 1024, 64, 4)  # hidden, inter, experts, top-k
+# ((hidden, inter, experts, top-k), group size, tokens, us of gate/up and down with the tiles, with the fold kernel).  Only
+# launches with a clear difference: the others may go either way.
+LAYERS = [
+    (FULL, 32, 64, (436, 278), (414, 198)), (FULL, 32, 2000, (3252, 1787), (2988, 1520)),
+    (FULL, 0, 48, (374, 213), (268, 151)), (SMALL, 0, 512, (104, 65), (83, 50)),
+    ((2048, 768, 16, 4), 32, 48, (34, 29), (50, 31)), ((2048, 256, 8, 2), 32, 64, (35, 19), (51, 25)),
+    ((2816, 128, 16, 8), 32, 128, (57, 30), (61, 34)), ((2560, 1600, 8, 1), 32, 48, (38, 34), (60, 44)),
+    ((1416, 616, 48, 6), 64, 301, (65, 45), (81, 44)),
+]
+
+
+def test_each_phase_of_a_layer_chooses_for_itself():
+    for (d, i, e, k), gs, m, tiles, fold in LAYERS:
+        got = hc.layer_route(d, i, gs, m, e, k)
+        for phase in (0, 1):
+            if abs(tiles[phase] - fold[phase]) > 0.03 * tiles[phase]:
+                assert got[phase] == ("fold" if fold[phase] < tiles[phase] else "tiles"), (d, i, gs, m, phase)
+    assert hc.layer_route(2048, 256, 0, 160, 100, 2) == ("fold", "tiles")     # one chunk of inter
+    assert hc.layer_route(1024, 2048, 0, 300, 36, 4) == ("tiles", "fold")    # four chunks of hidden
+
+
+def test_more_tokens_never_leave_the_fold_kernel():
+    # a layer's scratch is sized by the most tokens it has seen
+    for d, i, e, k in (FULL, SMALL, (2048, 256, 8, 2), (1416, 616, 48, 6), (3200, 1600, 100, 8), (2816, 128, 16, 8)):
+        for gs in (0, 32, 64, 128, 256):
+            seen = [False, False]
+            for m in list(range(3, 700)) + [1000, 2000, 3000, 4096, 8192]:
+                got = hc.layer_route(d, i, gs, m, e, k)
+                for phase in (0, 1):
+                    assert not (seen[phase] and got[phase] != "fold"), (d, i, e, k, gs, m, phase)
+                    seen[phase] |= got[phase] == "fold"
+
+
+def test_forced_layer_kernels_and_limits():
+    assert hc.layer_route(*FULL[:2], 32, 32, *FULL[2:]) == ("small", "small")
+    assert hc.layer_route(256, 96, 32, 4, 12, 3, want=2) == ("fold", "fold")
+    assert hc.layer_route(256, 96, 32, 4, 12, 3, want=1) == ("tiles", "tiles")
+    assert hc.layer_route(*FULL[:2], 32, 4096, *FULL[2:], want=0) == ("small", "small")
+    assert hc.layer_route(16385, 2048, 0, 512, 16, 4, want=2) == ("tiles", "fold")  # per-row rows too long for it
+    assert hc.layer_route(2048, 1024, 32, 4096, 1024, 8) == ("tiles", "tiles")      # 1025 slots: one too many

@@ -112,4 +112,34 @@ def test_wide_shared_expert_chooses_per_phase(dev, m, want_fold):
 
 def routed_folds(layer, m):
     """Launches of the routed experts that go to the fold kernel."""
-    return 2 if layer.hidden >= 2048 and m >= 48 and 2 * m * layer.k >= 3 * layer.n_experts else 0
+    return hc.layer_route(layer.hidden, layer.inter, layer.gs, m, layer.n_experts, layer.k).count("fold")
+
+
+@pytest.mark.parametrize("hidden,inter,m,experts,k,want", [
+    (2048, 256, 160, 100, 2, ("fold", "tiles")),   # one chunk of inter
+    (1024, 2048, 300, 36, 4, ("tiles", "fold")),   # four chunks of hidden
+])
+def test_layer_phases_on_different_kernels(dev, hidden, inter, m, experts, k, want):
+    assert hc.layer_route(hidden, inter, 0, m, experts, k) == want
+    layer = synth_layer(90 + k, hidden=hidden, inter=inter, n_experts=experts, k=k, gs=0, distinct_experts=3)
+    ml = upload_layer(dev, layer)
+    x = synth_tokens(91, m, hidden)
+    out = np.empty_like(x)
+    ml.forward(x, out)
+    got, n = fold_launches(dev, lambda: ml.forward(x, out))
+    assert n is None or n == 1
+    assert np.array_equal(bits(got), bits(oracle_layer_forward(layer, x, threads=8)))
+    assert cuda.last_device_error(dev) == 0
+    ml.free()
+
+
+def test_layer_with_few_items_stays_with_the_tiles(dev):
+    """Eight experts of 2048 x 256 give the fold kernel 18 gate/up items for 148 SMs (us: 35 with the tiles, 51)."""
+    layer = synth_layer(95, hidden=2048, inter=256, n_experts=8, k=2, gs=32, distinct_experts=2)
+    ml = upload_layer(dev, layer)
+    x = synth_tokens(96, 64, 2048)
+    ml.forward(x)
+    got, n = fold_launches(dev, lambda: ml.forward(x))
+    assert n is None or n == 0
+    assert np.array_equal(bits(got), bits(oracle_layer_forward(layer, x, threads=8)))
+    ml.free()

@@ -148,3 +148,11 @@ HC_API void pgb_hc_row_blocks(int rows, long long *out6) {
     out6[1] = R.narrow + R.wide;
     for (int g = 1; g <= 4; ++g) out6[1 + g] = R.units[g];
 }
+
+// The layer's choice for hidden D, inter I: bit 0 / 1 = fold kernel for gate/up / down, bit 2 / 3 = tiles.
+HC_API int pgb_hc_layer_route(int D, int I, int gs, int M, int E, int k, int sms, int want) {
+    W4Layout G, Dn;
+    if (!w4_layout_make(&G, I, D, gs != 0, gs) || !w4_layout_make(&Dn, D, I, gs != 0, gs)) return -1;
+    const LayerRoute r = layer_route(G, Dn, M, E, k, sms, want);
+    return (r.fold_gu ? 1 : 0) | (r.fold_dn ? 2 : 0) | (r.tiles_gu ? 4 : 0) | (r.tiles_dn ? 8 : 0);
+}
