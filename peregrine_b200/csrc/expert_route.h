@@ -49,8 +49,9 @@ struct RowBlocks {
 //   * small batch: units of 32 rows whose cost goes with their groups of 8 rows; cut finer when items are few.
 //     2048 x 4096, 64 rows: 28 us against 44.
 // Below 8 chunks of K and below 32 rows the small-batch kernel stays: nothing was settled there.
+inline bool fold_may_beat_block(const W4Layout &L, int max_rows) { return L.nchunk >= 8 && max_rows >= 32; }
 inline bool fold_beats_block(const W4Layout &L, int mode, const RowBlocks &R, int sms) {
-    if (!fold_fits(L, R.slots) || L.nchunk < 8 || R.max_rows < 32) return false;
+    if (!fold_fits(L, R.slots) || !fold_may_beat_block(L, R.max_rows)) return false;
     struct Cost {
         double fold, narrow, block;  // us per chunk and round; narrow items relative to wide ones
     };

@@ -143,3 +143,31 @@ def test_layer_with_few_items_stays_with_the_tiles(dev):
     assert n is None or n == 0
     assert np.array_equal(bits(got), bits(oracle_layer_forward(layer, x, threads=8)))
     ml.free()
+
+
+def test_fold_rows_take_no_scratch_of_their_own(dev):
+    """A layer's scratch for 8192 tokens is what the int8 layouts need, also where both phases take the fold kernel:
+    its fp16 rows lie in buffers that are idle at the time (their own would be 212 MB here)."""
+    import torch
+
+    hidden, inter, experts, k = 2048, 1024, 16, 8
+
+    def scratch(m):
+        pairs, kp, kpd = m * (k + 1), hidden, inter
+        return (pairs * (kp + kpd) * 17 // 16 + pairs * (kp + kpd) // 8 + pairs * 4 * (hidden + inter + 5)
+                + m * (kp + kp // 8 + hidden * 4 * 260 // 256 + 4 * experts + 16 * k))
+
+    layer = synth_layer(97, hidden=hidden, inter=inter, n_experts=experts, k=k, gs=32, distinct_experts=1)
+    ml = upload_layer(dev, layer, repeats="clone")
+    x = torch.randn(8192, hidden, device="cuda")
+    out = torch.empty_like(x)
+    torch.cuda.synchronize()
+    free = []
+    for m in (512, 8192):
+        assert hc.layer_route(hidden, inter, 32, m, experts, k) == ("fold", "fold")
+        ml.forward_dev(out.data_ptr(), x.data_ptr(), m)
+        assert cuda.lib().coli_cuda_pipe_sync(dev) == 1
+        free.append(cuda.mem_info(dev)[0])
+    grown, want = free[0] - free[1], scratch(8192) - scratch(512)
+    assert want - (64 << 20) < grown < want + (64 << 20), (grown, want)
+    ml.free()
