@@ -263,7 +263,8 @@ __global__ void __launch_bounds__(kBlkThreads, 1) gemv_w4a8_block_kernel(const G
 
     if (warp >= kBlkCW) {
         // ======================================================= producer warps
-        // Issuing a bulk copy costs the issuing warp ~130 cycles, one copy after the other; one warp
+        // Issuing a bulk copy under `lane == 0` costs the warp ~130 cycles (in part for the form of the
+        // condition, see elect_one in kernels_tcgen05.cuh), one copy after the other; one warp
         // issuing a stage's 18 copies took longer than the consumers needed for the stage.  So four
         // warps share them: producer p issues the chunks of tile pairs 2p and 2p + 1 (lanes 0-3: pair,
         // half), producer 0 also the item's activation rows and block sums, the byte count of the

@@ -26,10 +26,16 @@
 //                four blocks in tensor memory
 //   warp 12      one lane issues the MMAs: four per block (two halves, K = 16 each); dots of a group go to
 //                one of six accumulators of 64 columns
-//   warps 13, 14 bulk copies of the packed weight chunks (8 tiles each; issuing one costs ~130 cycles), a
-//                chunk of 256 elements per stage; warp 13 also takes work items from a device counter and
-//                publishes them to the other roles
+//   warps 13, 14 bulk copies of the packed weight chunks (8 tiles each), a chunk of 256 elements per stage; warp 13 also
+//                takes work items from a device counter and publishes them to the other roles
 //   warp 15      TMA tiles of the activations: fp16 rows, 64 elements x 32 rows, 128-byte swizzle
+//
+// Measured (B200): about 880 cycles per 32-element block of the 256 x 64 tile, epilogue included, against 256 of fold
+// arithmetic and 128 of MMA: a fold warp waits for a barrier, loads from tensor memory (60-80 cycles), waits and
+// folds, twice per block, and only two fold warps share a scheduler.  Issue slots 62 % busy, tensor pipe 16 %, DRAM
+// 4 % (1024 tokens, 16 experts of 6144 x 2048, group 32).  Layer of 256 such experts, 4096 tokens: 10.9 ms with the
+// mma.sync tiles, 10.0 ms here; 6144 x 32000 at 100 rows 199 us with the small-batch kernel, 169 us here.  Which
+// launches come here: expert_route.h.
 //
 // Persistent: one CTA per SM; the copies and MMAs of the next item run during an item's epilogue.  Items
 // are handed out heaviest first.  Every wait is bounded; one that runs out sets the device error word and
@@ -396,9 +402,8 @@ __global__ void __launch_bounds__(kFoThreads, 1)
                     for (int i = 0; i < CNT; ++i)
 #pragma unroll
                         for (int c = 0; c < 8; ++c) acc[h][i][c] = 0;
-            // One accumulator buffer of half h: its dots are folded in (grouped) or are the values themselves.
-                // Two groups are loaded before the first is used (a load
-                // takes ~60 cycles).
+                // One accumulator buffer of half h: its dots are folded in (grouped) or are the values themselves.
+                // Two groups are loaded before the first is used (a load takes 60-80 cycles).
                 auto drain_buf = [&](int h, float sc) {
                     um_spin(dfull + 8 * dp.i, dp.ph, fail);
                     tmem_fence_after();
@@ -464,7 +469,7 @@ __global__ void __launch_bounds__(kFoThreads, 1)
                     wp.next();
                 }
                 if (__any_sync(0xffffffffu, *fail)) return;
-            // ---- epilogue: lane = weight row, so the stores of a column are 128 consecutive bytes.  The
+                // ---- epilogue: lane = weight row, so the stores of a column are 128 consecutive bytes.  The
                 // column loops are rolled (registers are rotated under them): the body holds an fp64 exponential
                 // and unrolled over 64 columns it would be fetched from memory for every item.
                 const int l = 32 * q + lane;

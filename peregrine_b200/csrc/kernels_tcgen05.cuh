@@ -22,9 +22,9 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
 }
-// One thread of a converged warp.  Instructions whose operands live in uniform registers (MMA, commit, bulk and
-// tensor copies) compile to a loop over the active lanes under a condition like `lane == 0`: measured, an
-// MMA pair with its commits cost 165 cycles to issue that way and 34 in a block chosen by elect.sync.
+// One thread of a converged warp, chosen in the form that the compiler knows to be a single one: an MMA pair with its
+// commits takes 34 cycles to issue in a block chosen by elect.sync and 165 under a condition like `lane == 0`
+// (measured; bulk and tensor copies are of the same kind).
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -38,8 +38,7 @@ __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // try_wait that lets the hardware park the thread for up to `ns` nanoseconds instead of
-// returning at once: the waiting roles of this kernel share their schedulers with the fold warps
-// and must not spend issue slots on polling
+// returning at once (the peak probe, whose MMAs run for long)
 __device__ __forceinline__ uint32_t mbar_try_wait_park(uint32_t bar, uint32_t parity, uint32_t ns) {
     uint32_t ok;
     asm volatile(

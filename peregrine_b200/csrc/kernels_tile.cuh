@@ -216,7 +216,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) ffn_w4a8_tile_kernel(const Ge
 #pragma unroll
     for (int s = 0; s < 8; ++s) n_wt += wsrc[s] ? 1 : 0;
 
-    // A bulk copy holds the issuing warp for ~130 cycles, one copy after the other, so the ten copies
+    // A bulk copy issued under `lane == 0` holds the warp for ~130 cycles (in part for the form of the
+    // condition, see elect_one in kernels_tcgen05.cuh), one copy after the other, so the ten copies
     // of a stage are shared out: lane 0 of warp w issues weight tile w, warp 0 also sets the stage's
     // byte count, warps 1 and 2 also fetch the activation rows and their block sums.  (Copies of the
     // other warps may land before the count is set; the phase cannot complete before that arrival.)
