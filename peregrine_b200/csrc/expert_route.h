@@ -38,11 +38,27 @@ struct RowBlocks {
     }
 };
 
+// Rounds of a launch's items over `sms` CTAs that take the longest first: `wide` items of length 1, then `narrow` ones
+// of length w.
+inline double item_rounds(long long wide, long long narrow, double w, int sms) {
+    const long long late = wide % sms, early = sms - late;  // CTAs with one wide item more, and the others
+    const long long whole = narrow / sms > 4 ? narrow / sms - 4 : 0;
+    double a = (double)(wide / sms) + whole * w, b = a + 1.0;  // when they are free
+    double end = late ? b : a;
+    for (narrow -= whole * sms; narrow > 0;) {
+        const bool first = late == 0 || a <= b;
+        (first ? a : b) += w;
+        narrow -= first ? early : late;
+        if ((first ? a : b) > end) end = first ? a : b;
+    }
+    return end;
+}
+
 // Is the fold kernel faster than the shared-row small-batch kernel for these rows?  Both are given the time of
-// their rounds of items over the SMs.  The constants (us) are fitted to measured launches (B200; one matrix of K
-// 1536..6144, O 2048..33000 and 24..1200 rows, both phases of groups of 1..40 experts with up to 150 rows, five
-// formats).  Over the 1890 of them with 8+ chunks and 32+ rows the choice is 0.3 % behind the faster kernel of
-// each; 11 lose over 2 %, at most 12 %.
+// their rounds of items over the SMs.  The constants (us) are fitted to 7215 measured launches with 8+ chunks of K and
+// 32+ rows in some slot (B200; single matrices of O 200..33000 and K up to 6144 with up to 1200 rows, both phases
+// of groups of up to 40 experts with up to 150 rows, five formats).  Over these the choice is 0.1 % behind the faster
+// kernel of each; 44 lose over 2 %, at most 18 %.
 //   * fold: an item is 256 weight rows x up to 64 rows and always costs its whole width (or half of it); a last
 //     round that few items fill costs like a full one.  6144 x 16000, group 32: 128 rows 144 -> 97 us, 129 rows
 //     (three blocks of 43, 189 items) 145 against 170.
@@ -55,20 +71,21 @@ inline bool fold_beats_block(const W4Layout &L, int mode, const RowBlocks &R, in
     struct Cost {
         double fold, narrow, block;  // us per chunk and round; narrow items relative to wide ones
     };
-    const Cost per_row{1.80, 1.00, 2.15};
-    const Cost by_bpg[4] = {{3.20, 0.75, 2.25}, {2.60, 0.85, 2.05}, {2.15, 0.90, 2.05}, {1.90, 1.00, 2.05}};
+    const Cost per_row{1.75, 0.85, 2.05};
+    const Cost by_bpg[4] = {{3.20, 0.80, 2.30}, {2.60, 0.85, 2.15}, {2.05, 0.95, 2.30}, {1.90, 0.95, 2.20}};
     const Cost &c = !L.grouped ? per_row : by_bpg[L.bpg == 1 ? 0 : L.bpg == 2 ? 1 : L.bpg == 4 ? 2 : 3];
-    const double n_ob = mode == 0 ? (L.ntile + 7) / 8 : (L.ntile + 15) / 16;
-    const double chunks = L.nchunk + (mode == 0 ? 1.0 : 0.5);  // the epilogue, in chunks
-    const double items = n_ob * (R.narrow + R.wide), work = n_ob * (R.narrow * c.narrow + R.wide);
-    const double fold_rounds = items > sms ? work / sms + 0.4 * work / items : (R.wide ? 1.0 : c.narrow);
+    const long long n_ob = mode == 0 ? (L.ntile + 7) / 8 : (L.ntile + 15) / 16;
+    const double fold_rounds = item_rounds(n_ob * R.wide, n_ob * R.narrow, c.narrow, sms);
     double units = 0, weight = 0;
     for (int g = 1; g <= 4; ++g) {
-        units += n_ob * R.units[g];
-        weight += n_ob * R.units[g] * (0.28 + 0.18 * g);
+        units += (double)n_ob * R.units[g];
+        weight += (double)n_ob * R.units[g] * (0.12 + 0.22 * g);
     }
-    const double block_rounds = weight / sms + (units > sms ? 0.5 : 0.42);
-    return 18.0 + c.fold * chunks * fold_rounds < 14.0 + c.block * chunks * block_rounds;
+    const double block_rounds = weight / sms + (units > sms ? 0.45 : 0.42);
+    // (the epilogues count as chunks: gate/up's holds the SwiGLU)
+    const double fold_us = 17.0 + c.fold * (L.nchunk + (mode == 0 ? 1.5 : 0.0)) * fold_rounds;
+    const double block_us = 14.0 + c.block * (L.nchunk + (mode == 0 ? 2.0 : 0.5)) * block_rounds;
+    return fold_us < block_us;
 }
 
 // The same against the CTA-tiled mma.sync kernel, for one phase of a layer of M tokens, top-k of E experts, whose rows

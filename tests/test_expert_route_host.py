@@ -26,7 +26,8 @@ MEASURED = [
     (1, 16000, 3072, 32, [129], 79, 95), (1, 8192, 6144, 32, [129], 82, 95), (1, 8192, 6144, 32, [200], 136, 95),
     (1, 4096, 2048, 32, [64], 28, 44), (1, 33000, 6144, 32, [32], 92, 85), (1, 33000, 6144, 32, [1200], 1804, 1322),
     (1, 33000, 2048, 0, [32], 38, 32), (1, 16000, 6144, 0, [129], 135, 102), (1, 8192, 6144, 0, [32], 46, 58),
-    (1, 32000, 6144, 32, [100], 199, 172),
+    (1, 32000, 6144, 32, [100], 199, 172), (1, 10222, 4728, 32, [216], 113, 139), (1, 11116, 5192, 32, [203], 130, 150),
+    (1, 9822, 1808, 32, [229], 60, 72),
     (0, 1600, 4000, 32, RAMP40, 250, 311), (0, 2048, 6144, 32, RAMP40, 402, 499), (0, 1024, 2048, 32, RAMP40, 124, 146),
     (1, 6144, 2048, 32, RAMP40, 402, 451), (0, 1024, 2048, 32, [150] * 40, 475, 437), (0, 2048, 6144, 0, [28] * 39 + [32], 486, 403),
 ]
