@@ -96,12 +96,16 @@ inline bool fold_beats_block(const W4Layout &L, int mode, const RowBlocks &R, in
 // of 4 chunks 205 -> 192; where items are few (768 x 2048, 16 experts, 48 tokens: 102 items) 34 -> 50.  Per-row
 // scales, without a fold per group, are ahead from one round on (1600 x 2560, 8 experts, 200 tokens: 53 -> 47).  Below 8 chunks
 // gate/up, whose epilogue is the longer one, stays with the tiles (6 chunks group 64: 137 -> 146); grouped down of
-// one chunk too (58 -> 63).  Over all 611 layers the choice is 5.7 % ahead of the tiles alone and 0.4 % behind the
-// better kernel of each phase; 6 of them lose over 2 %, at most 8 %.
+// one chunk too (58 -> 63); so does gate/up whose blocks of 128 weight rows hold over a tenth more padding than the
+// tiles' of 64 (inter 136: layer of 1576 tokens 452 -> 502).  Over 2060 layers, 1449 of them drawn at random, the
+// choice is 5.1 % ahead of the tiles alone and 0.5 % behind the better kernel of each phase; 59 lose over 2 %, at most
+// 8 %.
 // (More tokens never take a layer back to the tiles: its scratch is sized by the most tokens it has seen.)
 inline bool fold_beats_tiles(const W4Layout &L, int mode, int M, int E, int k, int sms) {
     if (!fold_fits(L, E + 1) || L.nchunk < (mode == 0 ? 8 : L.grouped ? 2 : 1)) return false;
-    const double n_ob = mode == 0 ? (L.ntile + 7) / 8 : (L.ntile + 15) / 16;
+    const int ob = mode == 0 ? (L.ntile + 7) / 8 : (L.ntile + 15) / 16;
+    const double n_ob = ob;
+    if (mode == 0 && 20 * ob > 11 * ((L.ntile + 3) / 4)) return false;  // blocks of 128 rows against 64
     const double touched = E * (1.0 - std::pow(1.0 - (double)(k < E ? k : E) / E, M));
     const double full = (double)M * k / kFoTok;
     const double rounds = n_ob * ((touched > full ? touched : full) + (M + kFoTok - 1) / kFoTok) / sms;

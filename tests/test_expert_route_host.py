@@ -66,6 +66,9 @@ def test_each_phase_of_a_layer_chooses_for_itself():
             if abs(tiles[phase] - fold[phase]) > 0.03 * tiles[phase]:
                 assert got[phase] == ("fold" if fold[phase] < tiles[phase] else "tiles"), (d, i, gs, m, phase)
     assert hc.layer_route(2048, 256, 0, 160, 100, 2) == ("fold", "tiles")     # one chunk of inter
+    # 136 rows: two blocks of 128 against three of 64 (a layer of 452 us with the tiles, 502 with gate/up on the fold kernel)
+    assert hc.layer_route(2184, 136, 128, 1576, 40, 8) == ("tiles", "tiles")
+    assert hc.layer_route(2184, 256, 128, 1576, 40, 8) == ("fold", "tiles")
     assert hc.layer_route(1024, 2048, 0, 300, 36, 4) == ("tiles", "fold")    # four chunks of hidden
 
 
